@@ -11,9 +11,11 @@
 //                    on v, and the append of k and v to the (B, T, Hkv, D) cache: one warp per head.
 //   decode_attn      flash-decoding: grid (splits, heads, rows), each CTA reduces a slice of the visible
 //                    keys with an online softmax; the CTA that finishes last merges the slices.
+//   decode_qkv_attn  the two in one kernel, as the decode step runs them.
 // The reference does these steps with generic library ops (reference: nanochat/gpt.py:84-107,
 // nanochat/flash_attention.py:113-170 for the cached-attention call).
 #include "decode.h"
+#include "decode_attn.cuh"
 #include "host_utils.cuh"
 #include "ptx.cuh"
 
@@ -365,120 +367,134 @@ decode_qkv_post_kernel(__nv_bfloat16* __restrict__ qkv, long long ld, int H, int
 
 constexpr int kSplits = 8;
 
-// grid (kSplits, H, B), 128 threads. partial: (B, H, kSplits, 130) fp32 = [m, l, o[128]].
-__global__ void __launch_bounds__(128)
-decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long ldq, const __nv_bfloat16* __restrict__ k_cache,
-                   const __nv_bfloat16* __restrict__ v_cache, long long c_bat, long long c_tok,
-                   const int* __restrict__ seqlens, int H, int Hkv, int window, float scale_log2,
-                   float* __restrict__ partial, unsigned int* __restrict__ arrivals, __nv_bfloat16* __restrict__ y,
-                   long long ldy, KvPages pages) {
-  const int split = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int hkv = h / (H / Hkv);
-  // The row's page table does not change while a sequence is decoded (and the kernel before this one in the stream
-  // does not write it), so it is copied to shared memory before the wait on that kernel: the lookups of the key loop
-  // then cost a shared-memory read instead of a dependent global load in front of every key.
-  __shared__ int s_table[128];
-  if (pages.table != nullptr && pages.max_pages <= 128) {
-    if ((int)threadIdx.x < pages.max_pages) s_table[threadIdx.x] = pages.table[(long long)b * pages.max_pages + threadIdx.x];
-    pages.table = nullptr;
-    pages.max_pages = -1;                             // marks "table in shared memory" for the address helper below
+// What the attention kernel does about the step's own token. POST: the row of `qkv` still holds the projections; the CTA
+// turns and norms the query itself, and the CTA with the newest keys does the same to the new key (adding the value
+// embedding to the new value), attends to it from registers and appends both. Otherwise q is ready and the token is in
+// the cache.
+struct StepToken {
+  const __nv_bfloat16* cos_t; const __nv_bfloat16* sin_t;
+  const __nv_bfloat16* xn; long long ld_xn; const float* wg;         // value-embedding gate; xn == nullptr: none
+  const __nv_bfloat16* ve; long long ld_ve; const long long* idx;
+  int t_max; int* status;
+};
+
+// grid (splits, H, B), 256 threads. The splits of a row share its keys evenly; with more than one, each leaves
+// [m, l, o[128]] in `partial` and the one that arrives last merges them.
+// Bound by the dependent path position -> page -> key -> score -> weighted sum for a few rows, by L2 and HBM bytes for many
+// d26, 520 keys of 13 heads, B200: with a key per thread and a kernel of its own for the append 64 rows took 74 us and one
+// row 22.5; now 36.5 and 8.8.
+template <bool POST>
+__global__ void __launch_bounds__(kAttnWarps * 32)
+decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long ldq, __nv_bfloat16* __restrict__ k_cache,
+                   __nv_bfloat16* __restrict__ v_cache, long long c_bat, long long c_tok, const int* __restrict__ seqlens, int H,
+                   int Hkv, int window, float scale_log2, float* __restrict__ partial, unsigned int* __restrict__ arrivals,
+                   __nv_bfloat16* __restrict__ y, long long ldy, KvPages pages, StepToken tok) {
+  __shared__ AttnShared sh;
+  __shared__ int s_table[kTableCache];
+  __shared__ unsigned int s_last;
+  const int split = blockIdx.x, splits = gridDim.x, h = blockIdx.y, b = blockIdx.z, group = H / Hkv, hkv = h / group;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, hl = lane & 15;
+  // POST: positions, page table and older keys were there before the kernel in front of this one started (it makes the
+  // step's projections), so the first keys are requested before the wait on it. Else that kernel may write the cache.
+  if (!POST) { pdl_wait(); pdl_trigger(); }
+  const int pos = seqlens[b];
+  if (POST && (pos < 0 || pos >= tok.t_max)) {        // a full cache: record it and leave the row untouched
+    pdl_wait();
+    pdl_trigger();
+    if (tid == 0 && split == 0 && h == 0 && tok.status) atomicCAS(tok.status, 0, (ST_BAD_ARG << 24) | 0xdec0de);
+    return;
   }
-  auto token_offset = [&](int t) -> long long {
-    if (pages.max_pages == -1) {
-      return s_table[t >> pages.page_shift] * c_bat + (long long)(t & ((1 << pages.page_shift) - 1)) * c_tok;
-    }
-    return kv_token_offset(pages, b, t, c_bat, c_tok);
-  };
-  pdl_wait();
-  pdl_trigger();
-  const int pos = seqlens[b];                         // the new token sits at `pos`; it sees keys lo..pos
+  KvRow row = kv_row(pages, b, c_bat, c_tok);
+  if (row.table != nullptr && pages.max_pages <= kTableCache) {
+    if (tid < pages.max_pages) s_table[tid] = row.table[tid];
+    row.table = s_table;
+    __syncthreads();
+  }
   const int lo = window < 0 ? 0 : max(0, pos - window);
-  const int n_keys = pos - lo + 1;
-  const int chunk = (n_keys + kSplits - 1) / kSplits;
-  const int k_begin = lo + split * chunk;
-  const int k_end = min(pos + 1, k_begin + chunk);
-  // Two phases per tile of up to 128 keys: scores with one thread per key (no shuffles in the dot product),
-  // then the weighted sum of V with one thread per output dim (coalesced rows of V).
-  __shared__ float s_q[128];
-  __shared__ float s_p[128];
-  __shared__ float s_red[8];
-  __shared__ float s_o[4][128];
-  const int d = threadIdx.x;
-  s_q[d] = __bfloat162float(q[b * ldq + h * 128 + d]);
-  __syncthreads();
-  const __nv_bfloat16* kb = k_cache + hkv * 128;
-  const __nv_bfloat16* vb = v_cache + hkv * 128 + lane * 4;   // phase 2: a lane owns 4 dims
-  float M = -1.0e30f, L = 0.f, O = 0.f;
-  for (int tile = k_begin; tile < k_end; tile += 128) {
-    const int j = tile + d;
-    float sc = -1.0e30f;
-    if (j < k_end) {
-      const uint4* kr = reinterpret_cast<const uint4*>(kb + token_offset(j));
-      float acc = 0.f;
+  const int last = POST ? pos : pos + 1;              // one past the newest key in the cache
+  const int chunk = (last - lo + splits - 1) / splits;
+  const int begin = min(last, lo + split * chunk), end = min(last, begin + chunk);
+  const bool newest = split == splits - 1;
+  const __nv_bfloat16 *kb = k_cache + hkv * 128, *vb = v_cache + hkv * 128;
+  KeyBatch keys;
+  if (begin + 2 * warp < end) load_keys(keys, kb, vb, row, begin + 2 * warp, end);
+  if (POST) { pdl_wait(); pdl_trigger(); }
+  const __nv_bfloat16* proj = q + b * ldq;
+  uint4 qraw = *reinterpret_cast<const uint4*>(proj + h * 128 + hl * 8);
+  const __nv_bfloat16 *cos_p = nullptr, *sin_p = nullptr;
+  if (POST) {
+    cos_p = tok.cos_t + (long long)pos * 64;
+    sin_p = tok.sin_t + (long long)pos * 64;
+    qraw = rope_norm_half(qraw, cos_p, sin_p, hl);
+  }
+  float qf[8];
+  unpack8(qraw, qf);
+  HalfSoftmax st;
+  if (POST && newest && warp == kAttnWarps - 1) {
+    const uint4 kn = rope_norm_half(*reinterpret_cast<const uint4*>(proj + (H + hkv) * 128 + hl * 8), cos_p, sin_p, hl);
+    uint4 vn = *reinterpret_cast<const uint4*>(proj + (H + Hkv + hkv) * 128 + hl * 8);
+    if (tok.xn != nullptr) {
+      float g = hl < 12 ? __bfloat162float(tok.xn[b * tok.ld_xn + hl]) * tok.wg[hkv * 12 + hl] : 0.f;
+      g = 3.f / (1.f + __expf(-half_sum(g)));
+      float v[8], e[8];
+      unpack8(vn, v);
+      unpack8(*reinterpret_cast<const uint4*>(tok.ve + tok.idx[b] * tok.ld_ve + hkv * 128 + hl * 8), e);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const uint4 kv = kr[i];
-        const float2 k0 = unpack_bf16(kv.x), k1 = unpack_bf16(kv.y), k2 = unpack_bf16(kv.z), k3 = unpack_bf16(kv.w);
-        const float* qq = s_q + i * 8;
-        acc += k0.x * qq[0] + k0.y * qq[1] + k1.x * qq[2] + k1.y * qq[3] + k2.x * qq[4] + k2.y * qq[5] + k3.x * qq[6] +
-               k3.y * qq[7];
+      for (int i = 0; i < 8; ++i) v[i] += g * e[i];
+      vn = pack8(v);
+    }
+    float kf[8], vf[8], d = 0.f;
+    unpack8(kn, kf);
+    unpack8(vn, vf);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) d += qf[i] * kf[i];
+    const float s = half_sum(d) * scale_log2;
+    if (lane < 16) {                                  // the other half of the warp starts empty
+      st.m = s; st.l = 1.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) st.o[i] = vf[i];
+      if (h % group == 0) {
+        const long long o = row.at(pos) + hkv * 128 + hl * 8;
+        *reinterpret_cast<uint4*>(k_cache + o) = kn;
+        *reinterpret_cast<uint4*>(v_cache + o) = vn;
       }
-      sc = acc * scale_log2;
     }
-    float mx = sc;
-#pragma unroll
-    for (int w = 16; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
-    if (lane == 0) s_red[warp] = mx;
-    __syncthreads();
-    const float m_new = fmaxf(M, fmaxf(fmaxf(s_red[0], s_red[1]), fmaxf(s_red[2], s_red[3])));
-    const float pj = j < k_end ? exp2f(sc - m_new) : 0.f;
-    s_p[d] = pj;
-    const float ps = warp_sum(pj);
-    if (lane == 0) s_red[4 + warp] = ps;
-    __syncthreads();
-    const float alpha = exp2f(M - m_new);
-    L = L * alpha + (s_red[4] + s_red[5]) + (s_red[6] + s_red[7]);
-    // weighted sum of V: warp w takes keys w, w+4, ... (independent 8-byte loads, many in flight), then the four
-    // partial vectors are added per dim
-    const int cnt = min(128, k_end - tile);
-    float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
-#pragma unroll 8
-    for (int jj = warp; jj < cnt; jj += 4) {
-      const uint2 vr = *reinterpret_cast<const uint2*>(vb + token_offset(tile + jj));
-      const float2 v01 = unpack_bf16(vr.x), v23 = unpack_bf16(vr.y);
-      const float pw = s_p[jj];
-      o0 += pw * v01.x; o1 += pw * v01.y; o2 += pw * v23.x; o3 += pw * v23.y;
-    }
-    *reinterpret_cast<float4*>(&s_o[warp][lane * 4]) = make_float4(o0, o1, o2, o3);
-    __syncthreads();
-    O = O * alpha + (s_o[0][d] + s_o[1][d]) + (s_o[2][d] + s_o[3][d]);
-    M = m_new;
-    __syncthreads();                                   // s_p, s_o and s_red are rewritten by the next tile
+  }
+  attend_keys(st, keys, qf, kb, vb, row, begin, end, scale_log2);
+  leave_half(sh, st);
+  __syncthreads();
+  float m = 0.f, l = 0.f, o = 0.f;
+  if (tid < 128) merge_halves(sh, tid, m, l, o);
+  if (splits == 1) {
+    if (tid < 128) y[b * ldy + h * 128 + tid] = __float2bfloat16(l > 0.f ? o / l : 0.f);
+    return;
   }
   float* dst = partial + (((long long)b * H + h) * kSplits + split) * 130;
-  if (d == 0) { dst[0] = M; dst[1] = L; }
-  dst[2 + d] = O;
+  if (tid == 0) { dst[0] = m; dst[1] = l; }
+  if (tid < 128) dst[2 + tid] = o;
   // the split that arrives last merges all of them (the counter wraps back to zero by itself)
-  __shared__ unsigned int s_last;
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicInc(arrivals + b * H + h, kSplits - 1) == kSplits - 1;
+  if (tid == 0) s_last = atomicInc(arrivals + b * H + h, splits - 1) == splits - 1;
   __syncthreads();
-  if (!s_last) return;
+  if (!s_last || tid >= 128) return;
   __threadfence();
   const volatile float* src = partial + ((long long)b * H + h) * kSplits * 130;
-  float Mx = -1.0e30f;
-#pragma unroll
-  for (int s = 0; s < kSplits; ++s) Mx = fmaxf(Mx, src[s * 130]);
-  float Ls = 0.f, Os = 0.f;
-#pragma unroll
-  for (int s = 0; s < kSplits; ++s) {
+  float Mx = -1.0e30f, Ls = 0.f, Os = 0.f;
+  for (int s = 0; s < splits; ++s) Mx = fmaxf(Mx, src[s * 130]);
+  for (int s = 0; s < splits; ++s) {
     const float f = exp2f(src[s * 130] - Mx);
     Ls += f * src[s * 130 + 1];
-    Os += f * src[s * 130 + 2 + d];
+    Os += f * src[s * 130 + 2 + tid];
   }
-  y[b * ldy + h * 128 + d] = __float2bfloat16(Ls > 0.f ? Os / Ls : 0.f);
+  y[b * ldy + h * 128 + tid] = __float2bfloat16(Ls > 0.f ? Os / Ls : 0.f);
+}
+
+// Splits of a row's keys: as many as fill the chip once with two CTAs per SM, since a split costs a merge. One from
+// 23 rows of 13 heads on.
+int attn_splits(int B, int H) {
+  const int want = (2 * sm_count() + B * H - 1) / (B * H);
+  return want < 1 ? 1 : (want > kSplits ? kSplits : want);
 }
 
 }  // namespace
@@ -561,10 +577,29 @@ cudaError_t decode_attn(const void* q, long long ldq, const void* k_cache, const
                         float* scratch, void* y, long long ldy, const KvPages& pages, cudaStream_t s) {
   if (H % Hkv != 0) return cudaErrorInvalidValue;
   unsigned int* arrivals = reinterpret_cast<unsigned int*>(scratch + (size_t)B * H * kSplits * 130);
-  return launch_pdl(decode_attn_kernel, dim3(kSplits, H, B), dim3(128), s,
-      reinterpret_cast<const __nv_bfloat16*>(q), ldq, reinterpret_cast<const __nv_bfloat16*>(k_cache),
-      reinterpret_cast<const __nv_bfloat16*>(v_cache), c_bat, c_tok, seqlens, H, Hkv, window,
-      scale * 1.4426950408889634f, scratch, arrivals, reinterpret_cast<__nv_bfloat16*>(y), ldy, pages);
+  return launch_pdl(decode_attn_kernel<false>, dim3(attn_splits(B, H), H, B), dim3(kAttnWarps * 32), s,
+      reinterpret_cast<const __nv_bfloat16*>(q), ldq, reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(k_cache)),
+      reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(v_cache)), c_bat, c_tok, seqlens, H, Hkv, window,
+      scale * 1.4426950408889634f, scratch, arrivals, reinterpret_cast<__nv_bfloat16*>(y), ldy, pages, StepToken{});
+}
+
+cudaError_t decode_qkv_attn(const void* qkv, long long ld, void* k_cache, void* v_cache, long long c_bat, long long c_tok,
+                            const int* seqlens, int B, int H, int Hkv, int window, float scale, const void* cos_t,
+                            const void* sin_t, const void* xn, long long ld_xn, const float* wg, const void* ve,
+                            long long ld_ve, const long long* idx, int t_max, int* status, float* scratch, void* y,
+                            long long ldy, const KvPages& pages, cudaStream_t s) {
+  if (H % Hkv != 0 || ((ld | c_tok | ld_ve) & 7)) return cudaErrorInvalidValue;
+  if (pages.table != nullptr && (pages.page_shift < 0 || pages.page_shift > 16 || pages.max_pages <= 0 ||
+                                 t_max > (pages.max_pages << pages.page_shift)))
+    return cudaErrorInvalidValue;
+  unsigned int* arrivals = reinterpret_cast<unsigned int*>(scratch + (size_t)B * H * kSplits * 130);
+  const StepToken tok = {reinterpret_cast<const __nv_bfloat16*>(cos_t), reinterpret_cast<const __nv_bfloat16*>(sin_t),
+                         reinterpret_cast<const __nv_bfloat16*>(xn), ld_xn, wg, reinterpret_cast<const __nv_bfloat16*>(ve),
+                         ld_ve, idx, t_max, status};
+  return launch_pdl(decode_attn_kernel<true>, dim3(attn_splits(B, H), H, B), dim3(kAttnWarps * 32), s,
+      reinterpret_cast<const __nv_bfloat16*>(qkv), ld, reinterpret_cast<__nv_bfloat16*>(k_cache),
+      reinterpret_cast<__nv_bfloat16*>(v_cache), c_bat, c_tok, seqlens, H, Hkv, window, scale * 1.4426950408889634f, scratch,
+      arrivals, reinterpret_cast<__nv_bfloat16*>(y), ldy, pages, tok);
 }
 
 }  // namespace nc

@@ -169,7 +169,6 @@ class DecodeGraph(StepGraph):
     def _forward(self):
         m, C_ = self.model, self.C_
         B, H, Hkv = self.B, self.H, self.Hkv
-        nq = H * 128
         cache = self.cache
         idx = self.ids[:, 0]
         # embedding gather, norm, smear with the previous token's embedding and the update of that state: one kernel
@@ -193,13 +192,11 @@ class DecodeGraph(StepGraph):
             # a paged cache: one layer's page pools + the rows' page table; the row capacity bounds the append
             table = cache.table if self.paged else None
             t_max = cache.max_seq_len if self.paged else 0
-            C_.decode_qkv_post(self.qkv, H, Hkv, self.cos, self.sin, cache.cache_seqlens,
-                               self.xn if ve is not None else None, w["wg"] if ve is not None else None, ve,
-                               idx if ve is not None else None, kc, vc, table, t_max)
             window = m.window_sizes[i][0]
             window = window if 0 <= window < cache.max_seq_len else -1
-            C_.decode_attn(self.qkv[:, :nq], kc, vc, cache.cache_seqlens, H, Hkv, window, scale, self.scratch, self.y,
-                           table)
+            C_.decode_qkv_attn(self.qkv, H, Hkv, self.cos, self.sin, cache.cache_seqlens,
+                               self.xn if ve is not None else None, w["wg"] if ve is not None else None, ve,
+                               idx if ve is not None else None, kc, vc, window, scale, self.scratch, self.y, table, t_max)
             self._linear(self.y, w["o"], self.xa, aux=self.xm, next_w=w["fc"])
             self._linear(self.xa, w["fc"], self.h, relu2=True, norm_input=True, next_w=w["pr"])   # GEMV: norm(xa) folded in
             out = self.x_backout if i == backout_layer else self.xs[i & 1]
