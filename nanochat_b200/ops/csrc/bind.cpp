@@ -354,6 +354,49 @@ void gemv_rows_mix(const Tensor& x, const Tensor& x0, const Tensor& lam_r, const
                              (int)x.size(1), next_weights(next_w).first, next_weights(next_w).second, cur_stream()));
 }
 
+// x: (B, K), W: (N, K), out / aux: (B, N) bf16; x0, xm: (B, N) bf16 with lam_r, lam_0 fp32 (layers); xn: (B, K) bf16, its first
+// 16 channels are written; logits: fp32 (B, N).
+void rows_gemm(const Tensor& x, const Tensor& W, const optional<Tensor>& out, const optional<Tensor>& aux, bool relu2,
+               bool norm_input, const optional<Tensor>& x0, const optional<Tensor>& lam_r, const optional<Tensor>& lam_0,
+               int64_t layer, const optional<Tensor>& xm, const optional<Tensor>& xn, const optional<Tensor>& logits,
+               double softcap) {
+  auto has = [](const optional<Tensor>& t) { return t.has_value() && t->defined(); };
+  check_bf16(x, "x"); check_bf16(W, "W");
+  TORCH_CHECK(x.dim() == 2 && W.dim() == 2 && x.stride(1) == 1 && W.stride(1) == 1 && x.size(1) == W.size(1), "rows_gemm: x (B, K), W (N, K)");
+  const int64_t B = x.size(0), N = W.size(0), K = x.size(1);
+  auto rows = [&](const Tensor& t, const char* name) {
+    check_bf16(t, name);
+    TORCH_CHECK(t.dim() == 2 && t.size(0) == B && t.size(1) == N && t.stride(1) == 1, name, " must be (B, N) with unit column stride");
+  };
+  nc::RowsGemm g{};
+  g.x = x.data_ptr(); g.ldx = x.stride(0); g.W = W.data_ptr(); g.ldw = W.stride(0);
+  g.B = (int)B; g.N = (int)N; g.K = (int)K; g.norm_input = norm_input; g.relu2 = relu2;
+  if (has(out)) { rows(*out, "out"); g.out = out->data_ptr(); g.ldo = out->stride(0); }
+  if (has(aux)) { rows(*aux, "aux"); g.aux = aux->data_ptr(); g.ldaux = aux->stride(0); }
+  if (has(xm)) {
+    TORCH_CHECK(has(x0) && has(lam_r) && has(lam_0), "rows_gemm: xm needs x0, lam_r and lam_0");
+    rows(*xm, "xm"); rows(*x0, "x0");
+    TORCH_CHECK(lam_r->is_cuda() && lam_0->is_cuda() && lam_r->scalar_type() == at::kFloat && lam_0->scalar_type() == at::kFloat &&
+                lam_r->is_contiguous() && lam_0->is_contiguous() && layer >= 0 && layer < lam_r->numel() && layer < lam_0->numel(),
+                "lambdas: fp32 (layers)");
+    g.mix = {lam_r->data_ptr<float>(), lam_0->data_ptr<float>(), (int)layer, reinterpret_cast<const __nv_bfloat16*>(x0->data_ptr()),
+             x0->stride(0), reinterpret_cast<__nv_bfloat16*>(xm->data_ptr()), xm->stride(0)};
+  }
+  if (has(xn)) {
+    check_bf16(*xn, "xn");
+    TORCH_CHECK(norm_input && xn->sizes() == x.sizes() && xn->stride(1) == 1 && K >= 16 && N >= 16, "xn: like x, at least 16 wide");
+    g.xn_head = xn->data_ptr(); g.ldxn = xn->stride(0); g.head_cols = 16;
+  }
+  if (has(logits)) {
+    TORCH_CHECK(logits->is_cuda() && logits->scalar_type() == at::kFloat && logits->dim() == 2 && logits->size(0) == B &&
+                logits->size(1) == N && logits->stride(1) == 1, "logits: fp32 (B, N)");
+    g.logits = logits->data_ptr<float>(); g.ldl = logits->stride(0); g.softcap = (float)softcap;
+  }
+  const c10::cuda::CUDAGuard guard(x.device());
+  g.status = status_ptr(x);
+  NC_CHECK(nc::rows_gemm(g, cur_stream()));
+}
+
 // ids: int64 (B) or (B, 1); wte: (V, C) bf16; gate_w: fp32 (n_gate); lam: fp32 (1); prev, out: (B, C) bf16.
 void decode_embed(const Tensor& ids, const Tensor& wte, const Tensor& gate_w, const Tensor& lam, Tensor& prev, Tensor& out) {
   check_bf16(wte, "wte"); check_bf16(prev, "prev"); check_bf16(out, "out");
@@ -650,6 +693,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("norm_input"), py::arg("next_w") = py::none());
   m.def("gemv_rows_mix", &gemv_rows_mix, py::arg("x"), py::arg("x0"), py::arg("lam_r"), py::arg("lam_0"), py::arg("layer"),
         py::arg("W"), py::arg("out"), py::arg("xm"), py::arg("xn"), py::arg("next_w") = py::none());
+  m.def("rows_gemm", &rows_gemm, py::arg("x"), py::arg("W"), py::arg("out") = py::none(), py::arg("aux") = py::none(),
+        py::arg("relu2") = false, py::arg("norm_input") = false, py::arg("x0") = py::none(), py::arg("lam_r") = py::none(),
+        py::arg("lam_0") = py::none(), py::arg("layer") = 0, py::arg("xm") = py::none(), py::arg("xn") = py::none(),
+        py::arg("logits") = py::none(), py::arg("softcap") = 1.0);
   m.def("decode_embed", &decode_embed);
   m.def("decode_qkv_post", &decode_qkv_post, py::arg("qkv"), py::arg("H"), py::arg("Hkv"), py::arg("cos"), py::arg("sin"),
         py::arg("seqlens"), py::arg("xn"), py::arg("wg"), py::arg("ve"), py::arg("idx"), py::arg("k_cache"),

@@ -1,6 +1,7 @@
 // Host interface of the single-token decode kernels (decode.cu). All tensors bf16 unless noted; D = 128.
 #pragma once
 
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
 
@@ -33,6 +34,29 @@ cudaError_t gemv_rows_mix(const void* x, long long ldx, const void* x0, long lon
                           const float* lam_0, int layer, const void* W, long long ldw, void* out, long long ldo,
                           void* xm, long long ldxm, void* xn_head, long long ldxn, int head_cols, int B, int N, int K,
                           const void* next_w, long long next_bytes, cudaStream_t s);
+
+// The step's linear layers for up to kRowsGemmMax rows on tensor cores: y = epi(x' W^T) + aux, x' = x or rmsnorm(x)
+// (norm_input), epi = relu^2 where relu2. Any of three results, null for none: out (B x N) bf16; mix.xm = the next layer's
+// stream bf16(lam_r[layer] * bf16(y) + lam_0[layer] * x0); logits (B x N) fp32 = softcap * tanh(y / softcap).
+// xn_head: with norm_input, the first head_cols (<= 128) channels of rmsnorm(x). K, ldx, ldw multiples of 8, x and W
+// 16-byte aligned. W is read before the wait on the kernel in front, which must not be the one that wrote it.
+constexpr int kRowsGemmMax = 64;
+struct RowsMix {
+  const float* lam_r = nullptr; const float* lam_0 = nullptr; int layer = 0;
+  const __nv_bfloat16* x0 = nullptr; long long ldx0 = 0;
+  __nv_bfloat16* xm = nullptr; long long ldxm = 0;
+};
+struct RowsGemm {
+  const void* x; long long ldx; const void* W; long long ldw; int B, N, K;
+  int norm_input = 0, relu2 = 0;
+  const void* aux = nullptr; long long ldaux = 0;
+  void* out = nullptr; long long ldo = 0;
+  RowsMix mix;
+  void* xn_head = nullptr; long long ldxn = 0; int head_cols = 0;
+  float* logits = nullptr; long long ldl = 0; float softcap = 1.f;
+  int* status = nullptr;
+};
+cudaError_t rows_gemm(const RowsGemm& g, cudaStream_t s);
 
 // out[b] = e + lam * sigmoid(e[:n_gate] . gate_w) * prev[b], e = rmsnorm(wte[ids[b]]); prev[b] <- e. C, ldw, ldp, ldo
 // multiples of 8; n_gate <= 32; ids outside [0, vocab) are clamped.

@@ -4,8 +4,8 @@ Execution runtime: CUDA-graph replay of the single-token decode step.
 A decode step of the reference engine is one `model.forward` on a (B, 1) batch: a few hundred
 small library kernels whose launch cost, not their work, sets the token rate
 (reference: nanochat/engine.py:186-190). Here the step is a fixed sequence of purpose-built
-kernels (`ops/csrc/decode.cu`: weight-streaming GEMV with fused residual / relu^2, rotary +
-QK-norm + value-embedding gate + cache append, split-key attention) over static buffers. Every
+kernels (`ops/csrc/rows_gemm.cu`: linear layers of a few rows on tensor cores; `ops/csrc/decode.cu`: the same for one or two
+rows, rotary + QK-norm + value-embedding gate + cache append + split-key attention) over static buffers. Every
 position-dependent quantity is read from device memory (`KVCache.cache_seqlens`), so the whole
 step is captured once per (engine, cache) and replayed with a single launch per token.
 
@@ -24,13 +24,13 @@ from nanochat_b200 import common, ops
 from nanochat_b200.ops import reference as ref_ops
 
 LM_HEAD_PREFETCH_ROWS = 16384     # rows of lm_head (54 MB at 1664 wide) the last layer prefetches: what L2 can hold
-MAX_ROWS = 64          # rows of one decode graph; up to GEMV_ROWS of them use the weight-streaming GEMV
-GEMV_ROWS = 8
-# Up to this many rows the layer's mix + norm is folded into the QKV GEMV (one launch fewer per layer). Every CTA of
-# that GEMV redoes the mix for its rows, which is free while the kernel waits on memory (few rows) and costs more
-# than the launch it saves once the rows make it arithmetic-bound. Measured on d26: 1 row +4.8 %, 2 rows +2 %,
-# 4 rows -5 %, 8 rows -4 % tokens per second.
-FOLD_MIX_ROWS = int(os.environ.get("NANOCHAT_DECODE_FOLD_ROWS", "2"))
+MAX_ROWS = 64          # rows of one decode graph
+GEMV_ROWS = 8          # rows up to which the served families run their own step kernels
+# GPT's products: up to this many rows an fp32 matrix-vector kernel (mix and norm folded into the QKV product), from there on
+# the tensor-core kernel, whose chain is about a microsecond longer and does not grow with the rows. Measured per step, 512
+# tokens back: d26, 1 row 757 / 871 us, 2 rows 883 / 881, 4 rows 1399 / 1100, 8 rows 2046 / 1153; d12, 1 row 255 / 284,
+# 4 rows 356 / 326; d4, 1 row 83 / 86, 8 rows 166 / 106.
+VECTOR_ROWS = min(8, int(os.environ.get("NANOCHAT_DECODE_FOLD_ROWS", "2")))
 # every GEMV of the step prefetches the next kernel's weight matrix into L2 (NANOCHAT_DECODE_PREFETCH=0: off, A/B runs)
 PREFETCH_NEXT = os.environ.get("NANOCHAT_DECODE_PREFETCH", "1") != "0"
 
@@ -95,17 +95,17 @@ class DecodeGraph(StepGraph):
         bf16 = torch.bfloat16
         e = lambda *shape, dtype=bf16: torch.empty(*shape, dtype=dtype, device=dev)
         self.prev = torch.zeros(B, C, dtype=bf16, device=dev)
-        self.xm, self.xn, self.xa, self.xn2 = e(B, C), e(B, C), e(B, C), e(B, C)
+        self.xm, self.xn, self.xa = e(B, C), e(B, C), e(B, C)
         self.xs = [e(B, C), e(B, C)]                       # residual stream ping-pong
         self.x_in = e(B, C)                                # embedding + smear: the stream's input and the x0 of every layer
         self.x_backout = e(B, C)
         self.qkv, self.y, self.h = e(B, nq + 2 * nkv), e(B, nq), e(B, 4 * C)
-        self.logits_bf16 = e(B, model.lm_head.weight.shape[0])
         self.logits = e(B, cfg.vocab_size, dtype=torch.float32)
         self.scratch = torch.zeros(self.C_.decode_attn_scratch(B, self.H), dtype=torch.float32, device=dev)
         self.cos = model.cos.reshape(-1, 64).contiguous()
         self.sin = model.sin.reshape(-1, 64).contiguous()
-        self.use_gemv = B <= GEMV_ROWS     # more rows: the tcgen05 GEMM (rows padded to a 128-row tile) inside the graph
+        self.vector = B <= VECTOR_ROWS
+        self.logits_bf16 = e(B, model.lm_head.weight.shape[0]) if self.vector else None
         self.weights_epoch = None
         self.w = None
 
@@ -152,19 +152,11 @@ class DecodeGraph(StepGraph):
         self._captured_where = where
 
     # --------------------------------------------------------------------- step
-    def _linear(self, x, w, out, aux=None, relu2=False, norm_input=False, next_w=None):
-        """out = epi(norm?(x) @ w^T) (+ aux): GEMV for a few rows, tensor-core GEMM otherwise. `next_w`: the weight
-        matrix the following kernel will stream; the GEMV's CTAs prefetch it into L2 (decode is latency-bound per
-        kernel, so keeping HBM busy across kernel boundaries is what raises the weight-streaming rate)."""
-        if self.use_gemv:
-            self.C_.gemv_rows(x, w, out, aux, 1 if relu2 else 0, norm_input, next_w if PREFETCH_NEXT else None)
-            return
-        nat = self.nat
-        if norm_input:
-            self.C_.norm_fwd(x, self.xn2, None)
-            x = self.xn2
-        nat.gemm(x, w, out, aux=aux, beta=1.0 if aux is not None else 0.0,
-                 epi=nat.EPI_RELU2 if relu2 else nat.EPI_LINEAR)
+    def _gemv(self, x, w, out, aux=None, relu2=False, norm_input=False, next_w=None):
+        """out = epi(norm?(x) @ w^T) (+ aux). `next_w`: the weight matrix the following kernel will stream; the GEMV's CTAs
+        prefetch it into L2 (decode is latency-bound per kernel, so keeping HBM busy across kernel boundaries is what raises
+        the weight-streaming rate)."""
+        self.C_.gemv_rows(x, w, out, aux, 1 if relu2 else 0, norm_input, next_w if PREFETCH_NEXT else None)
 
     def _forward(self):
         m, C_ = self.model, self.C_
@@ -178,15 +170,15 @@ class DecodeGraph(StepGraph):
         backout_layer = m.config.n_layer // 2
         scale = 1.0 / (128 ** 0.5)
         for i, w in enumerate(self.w):
-            # what the kernel after this layer's last GEMV streams: the next layer's QKV weights, or the head of lm_head
-            after = self.w[i + 1]["qkv"] if i + 1 < len(self.w) else self.lm_head[:LM_HEAD_PREFETCH_ROWS]
-            if self.use_gemv and B <= FOLD_MIX_ROWS:
+            last = i + 1 == len(self.w)
+            if self.vector:
                 # mix + norm folded into the QKV GEMV; its first CTA writes xm and the gate's slice of xn
                 C_.gemv_rows_mix(x, x0, m.resid_lambdas, m.x0_lambdas, i, w["qkv"], self.qkv, self.xm, self.xn,
                                  w["o"] if PREFETCH_NEXT else None)
             else:
-                C_.mixnorm_fwd(x, x0, m.resid_lambdas, m.x0_lambdas, i, self.xm, self.xn, None)
-                self._linear(self.xn, w["qkv"], self.qkv, next_w=w["o"])
+                if i == 0:                       # later layers: the MLP's last product leaves the next layer's mix
+                    C_.mixnorm_fwd(x, x0, m.resid_lambdas, m.x0_lambdas, 0, self.xm, self.xn, None)
+                C_.rows_gemm(self.xm, w["qkv"], self.qkv, norm_input=True, xn=self.xn if w["wg"] is not None else None)
             ve = m.value_embeds[str(i)].weight if str(i) in m.value_embeds else None
             kc, vc = cache.get_layer_cache(i)
             # a paged cache: one layer's page pools + the rows' page table; the row capacity bounds the append
@@ -197,14 +189,25 @@ class DecodeGraph(StepGraph):
             C_.decode_qkv_attn(self.qkv, H, Hkv, self.cos, self.sin, cache.cache_seqlens,
                                self.xn if ve is not None else None, w["wg"] if ve is not None else None, ve,
                                idx if ve is not None else None, kc, vc, window, scale, self.scratch, self.y, table, t_max)
-            self._linear(self.y, w["o"], self.xa, aux=self.xm, next_w=w["fc"])
-            self._linear(self.xa, w["fc"], self.h, relu2=True, norm_input=True, next_w=w["pr"])   # GEMV: norm(xa) folded in
             out = self.x_backout if i == backout_layer else self.xs[i & 1]
-            self._linear(self.h, w["pr"], out, aux=self.xa, next_w=after)
+            if self.vector:
+                # what the kernel after this layer's last GEMV streams: the next layer's QKV weights, or the head of lm_head
+                after = self.lm_head[:LM_HEAD_PREFETCH_ROWS] if last else self.w[i + 1]["qkv"]
+                self._gemv(self.y, w["o"], self.xa, aux=self.xm, next_w=w["fc"])
+                self._gemv(self.xa, w["fc"], self.h, relu2=True, norm_input=True, next_w=w["pr"])
+                self._gemv(self.h, w["pr"], out, aux=self.xa, next_w=after)
+            else:
+                C_.rows_gemm(self.y, w["o"], self.xa, self.xm)
+                C_.rows_gemm(self.xa, w["fc"], self.h, relu2=True, norm_input=True)
+                mix = {} if last else dict(x0=x0, lam_r=m.resid_lambdas, lam_0=m.x0_lambdas, layer=i + 1, xm=self.xm)
+                C_.rows_gemm(self.h, w["pr"], out if last or i == backout_layer else None, self.xa, **mix)
             x = out
         C_.backout_norm_fwd(x, self.x_backout, m.backout_lambda.detach().float(), self.xn)
-        self._linear(self.xn, self.lm_head, self.logits_bf16)
-        C_.softcap_logits(self.logits_bf16, self.logits, m.config.vocab_size, ref_ops.SOFTCAP)
+        if self.vector:
+            self._gemv(self.xn, self.lm_head, self.logits_bf16)
+            C_.softcap_logits(self.logits_bf16, self.logits, m.config.vocab_size, ref_ops.SOFTCAP)
+        else:
+            C_.rows_gemm(self.xn, self.lm_head[:m.config.vocab_size], logits=self.logits, softcap=ref_ops.SOFTCAP)
         cache.cache_seqlens.add_(1)
 
     def begin(self):

@@ -92,6 +92,32 @@ def test_gemv_with_folded_mix_and_norm_matches_the_separate_kernels():
     nat.check_status()
 
 
+@pytest.mark.parametrize("B,N,K", [(1, 128, 8), (1, 4992, 1664), (3, 520, 6656), (16, 1000, 72), (17, 1664, 6656), (32, 129, 256),
+                                   (33, 2304, 768), (64, 6656, 1664), (64, 32768, 512)])
+def test_rows_gemm_matches_fp32(B, N, K):
+    from nanochat_b200.ops import native as nat
+    g = torch.Generator(device="cuda").manual_seed(B + N)
+    x = torch.randn(B, K, device="cuda", generator=g).to(BF16)
+    W = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).to(BF16)
+    aux, x0 = (torch.randn(B, N, device="cuda", generator=g).to(BF16) for _ in range(2))
+    lam_r, lam_0 = torch.tensor([1.0, 0.9], device="cuda"), torch.tensor([0.0, 0.2], device="cuda")
+    out, xm, xn = torch.empty(B, N, dtype=BF16, device="cuda"), torch.empty(B, N, dtype=BF16, device="cuda"), torch.zeros_like(x)
+    logits = torch.empty(B, N, device="cuda")
+    ref, xf = x.float() @ W.float().t(), x.float()
+    close = lambda a, b: ((a.float() - b).norm() / b.norm()).item() < 4e-3          # a bf16 result is off by at most 2^-9 = 2e-3
+    nat._C.rows_gemm(x, W, out, aux, relu2=True, x0=x0, lam_r=lam_r, lam_0=lam_0, layer=1, xm=xm)
+    assert close(out, torch.relu(ref) ** 2 + aux.float())
+    assert close(xm, 0.9 * out.float() + 0.2 * x0.float())
+    nat._C.rows_gemm(x, W, logits=logits, softcap=15.0)
+    assert ((logits - 15 * torch.tanh(ref / 15)).norm() / ref.norm()).item() < 1e-5
+    rstd = torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1.1920929e-07)
+    nat._C.rows_gemm(x, W, out, norm_input=True, xn=xn if K >= 16 else None)
+    assert close(out, rstd * ref)
+    if K >= 16:
+        assert close(xn[:, :16], (rstd * xf)[:, :16]) and xn[:, 16:].abs().sum().item() == 0
+    nat.check_status()
+
+
 def test_decode_embed_matches_fp32():
     from nanochat_b200.ops import native as nat
     g = torch.Generator(device="cuda").manual_seed(11)
