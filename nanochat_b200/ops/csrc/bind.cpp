@@ -474,8 +474,8 @@ void decode_attn(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, 
 // decode_qkv_post and decode_attn in one launch; arguments as there (qkv is left as it is).
 void decode_qkv_attn(const Tensor& qkv, int64_t H, int64_t Hkv, const Tensor& cos_t, const Tensor& sin_t, const Tensor& seqlens,
                      const optional<Tensor>& xn, const optional<Tensor>& wg, const optional<Tensor>& ve,
-                     const optional<Tensor>& idx, Tensor& k_cache, Tensor& v_cache, int64_t window, double scale, Tensor& scratch,
-                     Tensor& y, const optional<Tensor>& table, int64_t t_max) {
+                     const optional<Tensor>& idx, Tensor& k_cache, Tensor& v_cache, int64_t window, double scale, Tensor& y,
+                     const optional<Tensor>& table, int64_t t_max) {
   check_bf16(qkv, "qkv"); check_bf16(cos_t, "cos"); check_bf16(sin_t, "sin"); check_bf16(k_cache, "k_cache");
   check_bf16(v_cache, "v_cache"); check_bf16(y, "y");
   TORCH_CHECK(qkv.dim() == 2 && qkv.stride(1) == 1 && qkv.size(1) == (H + 2 * Hkv) * 128, "qkv shape");
@@ -486,8 +486,6 @@ void decode_qkv_attn(const Tensor& qkv, int64_t H, int64_t Hkv, const Tensor& co
   TORCH_CHECK(k_cache.dim() == 4 && (paged || k_cache.size(0) == qkv.size(0)) && k_cache.size(2) == Hkv &&
               k_cache.size(3) == 128 && k_cache.stride(3) == 1 && k_cache.stride(2) == 128 &&
               v_cache.strides() == k_cache.strides(), "cache layout");
-  TORCH_CHECK(scratch.scalar_type() == at::kFloat &&
-              (size_t)scratch.numel() >= nc::decode_attn_scratch_floats((int)qkv.size(0), (int)H), "scratch too small");
   const nc::KvPages pages = kv_pages(table, k_cache, qkv.size(0));
   const bool has_ve = ve.has_value() && ve->defined();
   if (has_ve) {
@@ -500,8 +498,7 @@ void decode_qkv_attn(const Tensor& qkv, int64_t H, int64_t Hkv, const Tensor& co
                                cos_t.data_ptr(), sin_t.data_ptr(), has_ve ? xn->data_ptr() : nullptr, has_ve ? xn->stride(0) : 0,
                                has_ve ? wg->data_ptr<float>() : nullptr, has_ve ? ve->data_ptr() : nullptr,
                                has_ve ? ve->stride(0) : 0, has_ve ? reinterpret_cast<const long long*>(idx->data_ptr<int64_t>()) : nullptr,
-                               (int)(paged ? t_max : k_cache.size(1)), status_ptr(qkv), scratch.data_ptr<float>(), y.data_ptr(),
-                               y.stride(0), pages, cur_stream()));
+                               (int)(paged ? t_max : k_cache.size(1)), status_ptr(qkv), y.data_ptr(), y.stride(0), pages, cur_stream()));
 }
 int64_t decode_attn_scratch(int64_t B, int64_t H) { return (int64_t)nc::decode_attn_scratch_floats((int)B, (int)H); }
 
@@ -705,7 +702,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("Hkv"), py::arg("window"), py::arg("scale"), py::arg("scratch"), py::arg("y"), py::arg("table") = py::none());
   m.def("decode_qkv_attn", &decode_qkv_attn, py::arg("qkv"), py::arg("H"), py::arg("Hkv"), py::arg("cos"), py::arg("sin"),
         py::arg("seqlens"), py::arg("xn"), py::arg("wg"), py::arg("ve"), py::arg("idx"), py::arg("k_cache"), py::arg("v_cache"),
-        py::arg("window"), py::arg("scale"), py::arg("scratch"), py::arg("y"), py::arg("table") = py::none(), py::arg("t_max") = 0);
+        py::arg("window"), py::arg("scale"), py::arg("y"), py::arg("table") = py::none(), py::arg("t_max") = 0);
   m.def("decode_attn_scratch", &decode_attn_scratch);
   m.def("amax_bf16", &amax_bf16);
   m.def("quantize_bf16", &quantize_bf16, py::arg("x"), py::arg("amax"), py::arg("q"), py::arg("inv_scale"),

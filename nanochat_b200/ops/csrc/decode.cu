@@ -11,7 +11,7 @@
 //                    on v, and the append of k and v to the (B, T, Hkv, D) cache: one warp per head.
 //   decode_attn      flash-decoding: grid (splits, heads, rows), each CTA reduces a slice of the visible
 //                    keys with an online softmax; the CTA that finishes last merges the slices.
-//   decode_qkv_attn  the two in one kernel, as the decode step runs them.
+//   decode_qkv_attn  the two in one kernel, as the decode step runs them (decode_attn.cu).
 // The reference does these steps with generic library ops (reference: nanochat/gpt.py:84-107,
 // nanochat/flash_attention.py:113-170 for the cached-attention call).
 #include "decode.h"
@@ -367,43 +367,21 @@ decode_qkv_post_kernel(__nv_bfloat16* __restrict__ qkv, long long ld, int H, int
 
 constexpr int kSplits = 8;
 
-// What the attention kernel does about the step's own token. POST: the row of `qkv` still holds the projections; the CTA
-// turns and norms the query itself, and the CTA with the newest keys does the same to the new key (adding the value
-// embedding to the new value), attends to it from registers and appends both. Otherwise q is ready and the token is in
-// the cache.
-struct StepToken {
-  const __nv_bfloat16* cos_t; const __nv_bfloat16* sin_t;
-  const __nv_bfloat16* xn; long long ld_xn; const float* wg;         // value-embedding gate; xn == nullptr: none
-  const __nv_bfloat16* ve; long long ld_ve; const long long* idx;
-  int t_max; int* status;
-};
-
 // grid (splits, H, B), 256 threads. The splits of a row share its keys evenly; with more than one, each leaves
 // [m, l, o[128]] in `partial` and the one that arrives last merges them.
-// Bound by the dependent path position -> page -> key -> score -> weighted sum for a few rows, by L2 and HBM bytes for many
-// d26, 520 keys of 13 heads, B200: with a key per thread and a kernel of its own for the append 64 rows took 74 us and one
-// row 22.5; now 36.5 and 8.8.
-template <bool POST>
 __global__ void __launch_bounds__(kAttnWarps * 32)
-decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long ldq, __nv_bfloat16* __restrict__ k_cache,
-                   __nv_bfloat16* __restrict__ v_cache, long long c_bat, long long c_tok, const int* __restrict__ seqlens, int H,
+decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long ldq, const __nv_bfloat16* __restrict__ k_cache,
+                   const __nv_bfloat16* __restrict__ v_cache, long long c_bat, long long c_tok, const int* __restrict__ seqlens, int H,
                    int Hkv, int window, float scale_log2, float* __restrict__ partial, unsigned int* __restrict__ arrivals,
-                   __nv_bfloat16* __restrict__ y, long long ldy, KvPages pages, StepToken tok) {
+                   __nv_bfloat16* __restrict__ y, long long ldy, KvPages pages) {
   __shared__ AttnShared sh;
   __shared__ int s_table[kTableCache];
   __shared__ unsigned int s_last;
   const int split = blockIdx.x, splits = gridDim.x, h = blockIdx.y, b = blockIdx.z, group = H / Hkv, hkv = h / group;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, hl = lane & 15;
-  // POST: positions, page table and older keys were there before the kernel in front of this one started (it makes the
-  // step's projections), so the first keys are requested before the wait on it. Else that kernel may write the cache.
-  if (!POST) { pdl_wait(); pdl_trigger(); }
+  pdl_wait();
+  pdl_trigger();
   const int pos = seqlens[b];
-  if (POST && (pos < 0 || pos >= tok.t_max)) {        // a full cache: record it and leave the row untouched
-    pdl_wait();
-    pdl_trigger();
-    if (tid == 0 && split == 0 && h == 0 && tok.status) atomicCAS(tok.status, 0, (ST_BAD_ARG << 24) | 0xdec0de);
-    return;
-  }
   KvRow row = kv_row(pages, b, c_bat, c_tok);
   if (row.table != nullptr && pages.max_pages <= kTableCache) {
     if (tid < pages.max_pages) s_table[tid] = row.table[tid];
@@ -411,55 +389,15 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long ldq, __nv_bflo
     __syncthreads();
   }
   const int lo = window < 0 ? 0 : max(0, pos - window);
-  const int last = POST ? pos : pos + 1;              // one past the newest key in the cache
+  const int last = pos + 1;                           // one past the newest key in the cache
   const int chunk = (last - lo + splits - 1) / splits;
   const int begin = min(last, lo + split * chunk), end = min(last, begin + chunk);
-  const bool newest = split == splits - 1;
   const __nv_bfloat16 *kb = k_cache + hkv * 128, *vb = v_cache + hkv * 128;
   KeyBatch keys;
   if (begin + 2 * warp < end) load_keys(keys, kb, vb, row, begin + 2 * warp, end);
-  if (POST) { pdl_wait(); pdl_trigger(); }
-  const __nv_bfloat16* proj = q + b * ldq;
-  uint4 qraw = *reinterpret_cast<const uint4*>(proj + h * 128 + hl * 8);
-  const __nv_bfloat16 *cos_p = nullptr, *sin_p = nullptr;
-  if (POST) {
-    cos_p = tok.cos_t + (long long)pos * 64;
-    sin_p = tok.sin_t + (long long)pos * 64;
-    qraw = rope_norm_half(qraw, cos_p, sin_p, hl);
-  }
   float qf[8];
-  unpack8(qraw, qf);
+  unpack8(*reinterpret_cast<const uint4*>(q + b * ldq + h * 128 + hl * 8), qf);
   HalfSoftmax st;
-  if (POST && newest && warp == kAttnWarps - 1) {
-    const uint4 kn = rope_norm_half(*reinterpret_cast<const uint4*>(proj + (H + hkv) * 128 + hl * 8), cos_p, sin_p, hl);
-    uint4 vn = *reinterpret_cast<const uint4*>(proj + (H + Hkv + hkv) * 128 + hl * 8);
-    if (tok.xn != nullptr) {
-      float g = hl < 12 ? __bfloat162float(tok.xn[b * tok.ld_xn + hl]) * tok.wg[hkv * 12 + hl] : 0.f;
-      g = 3.f / (1.f + __expf(-half_sum(g)));
-      float v[8], e[8];
-      unpack8(vn, v);
-      unpack8(*reinterpret_cast<const uint4*>(tok.ve + tok.idx[b] * tok.ld_ve + hkv * 128 + hl * 8), e);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] += g * e[i];
-      vn = pack8(v);
-    }
-    float kf[8], vf[8], d = 0.f;
-    unpack8(kn, kf);
-    unpack8(vn, vf);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) d += qf[i] * kf[i];
-    const float s = half_sum(d) * scale_log2;
-    if (lane < 16) {                                  // the other half of the warp starts empty
-      st.m = s; st.l = 1.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) st.o[i] = vf[i];
-      if (h % group == 0) {
-        const long long o = row.at(pos) + hkv * 128 + hl * 8;
-        *reinterpret_cast<uint4*>(k_cache + o) = kn;
-        *reinterpret_cast<uint4*>(v_cache + o) = vn;
-      }
-    }
-  }
   attend_keys(st, keys, qf, kb, vb, row, begin, end, scale_log2);
   leave_half(sh, st);
   __syncthreads();
@@ -577,29 +515,10 @@ cudaError_t decode_attn(const void* q, long long ldq, const void* k_cache, const
                         float* scratch, void* y, long long ldy, const KvPages& pages, cudaStream_t s) {
   if (H % Hkv != 0) return cudaErrorInvalidValue;
   unsigned int* arrivals = reinterpret_cast<unsigned int*>(scratch + (size_t)B * H * kSplits * 130);
-  return launch_pdl(decode_attn_kernel<false>, dim3(attn_splits(B, H), H, B), dim3(kAttnWarps * 32), s,
-      reinterpret_cast<const __nv_bfloat16*>(q), ldq, reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(k_cache)),
-      reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(v_cache)), c_bat, c_tok, seqlens, H, Hkv, window,
-      scale * 1.4426950408889634f, scratch, arrivals, reinterpret_cast<__nv_bfloat16*>(y), ldy, pages, StepToken{});
-}
-
-cudaError_t decode_qkv_attn(const void* qkv, long long ld, void* k_cache, void* v_cache, long long c_bat, long long c_tok,
-                            const int* seqlens, int B, int H, int Hkv, int window, float scale, const void* cos_t,
-                            const void* sin_t, const void* xn, long long ld_xn, const float* wg, const void* ve,
-                            long long ld_ve, const long long* idx, int t_max, int* status, float* scratch, void* y,
-                            long long ldy, const KvPages& pages, cudaStream_t s) {
-  if (H % Hkv != 0 || ((ld | c_tok | ld_ve) & 7)) return cudaErrorInvalidValue;
-  if (pages.table != nullptr && (pages.page_shift < 0 || pages.page_shift > 16 || pages.max_pages <= 0 ||
-                                 t_max > (pages.max_pages << pages.page_shift)))
-    return cudaErrorInvalidValue;
-  unsigned int* arrivals = reinterpret_cast<unsigned int*>(scratch + (size_t)B * H * kSplits * 130);
-  const StepToken tok = {reinterpret_cast<const __nv_bfloat16*>(cos_t), reinterpret_cast<const __nv_bfloat16*>(sin_t),
-                         reinterpret_cast<const __nv_bfloat16*>(xn), ld_xn, wg, reinterpret_cast<const __nv_bfloat16*>(ve),
-                         ld_ve, idx, t_max, status};
-  return launch_pdl(decode_attn_kernel<true>, dim3(attn_splits(B, H), H, B), dim3(kAttnWarps * 32), s,
-      reinterpret_cast<const __nv_bfloat16*>(qkv), ld, reinterpret_cast<__nv_bfloat16*>(k_cache),
-      reinterpret_cast<__nv_bfloat16*>(v_cache), c_bat, c_tok, seqlens, H, Hkv, window, scale * 1.4426950408889634f, scratch,
-      arrivals, reinterpret_cast<__nv_bfloat16*>(y), ldy, pages, tok);
+  return launch_pdl(decode_attn_kernel, dim3(attn_splits(B, H), H, B), dim3(kAttnWarps * 32), s,
+      reinterpret_cast<const __nv_bfloat16*>(q), ldq, reinterpret_cast<const __nv_bfloat16*>(k_cache),
+      reinterpret_cast<const __nv_bfloat16*>(v_cache), c_bat, c_tok, seqlens, H, Hkv, window,
+      scale * 1.4426950408889634f, scratch, arrivals, reinterpret_cast<__nv_bfloat16*>(y), ldy, pages);
 }
 
 }  // namespace nc

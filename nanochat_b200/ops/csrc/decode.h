@@ -82,12 +82,12 @@ cudaError_t decode_attn(const void* q, long long ldq, const void* k_cache, const
                         float* scratch, void* y, long long ldy, const KvPages& pages, cudaStream_t s);
 
 // decode_qkv_post and decode_attn in one kernel on unchanged projections (B rows of [q heads | k heads | v heads]): the
-// arithmetic, roundings, append and full-cache rule of the two. Row pitches multiples of 8. Positions, page table and the
+// arithmetic, roundings, append and full-cache rule of the two. Row and page pitches multiples of 8. Positions, page table and the
 // tokens before the step's own are read before the wait on the kernel in front, which must not be the one that wrote them.
 cudaError_t decode_qkv_attn(const void* qkv, long long ld, void* k_cache, void* v_cache, long long c_bat, long long c_tok,
                             const int* seqlens, int B, int H, int Hkv, int window, float scale, const void* cos_t,
                             const void* sin_t, const void* xn, long long ld_xn, const float* wg, const void* ve,
-                            long long ld_ve, const long long* idx, int t_max, int* status, float* scratch, void* y,
-                            long long ldy, const KvPages& pages, cudaStream_t s);
+                            long long ld_ve, const long long* idx, int t_max, int* status, void* y, long long ldy,
+                            const KvPages& pages, cudaStream_t s);
 
 }  // namespace nc

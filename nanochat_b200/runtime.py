@@ -101,7 +101,6 @@ class DecodeGraph(StepGraph):
         self.x_backout = e(B, C)
         self.qkv, self.y, self.h = e(B, nq + 2 * nkv), e(B, nq), e(B, 4 * C)
         self.logits = e(B, cfg.vocab_size, dtype=torch.float32)
-        self.scratch = torch.zeros(self.C_.decode_attn_scratch(B, self.H), dtype=torch.float32, device=dev)
         self.cos = model.cos.reshape(-1, 64).contiguous()
         self.sin = model.sin.reshape(-1, 64).contiguous()
         self.vector = B <= VECTOR_ROWS
@@ -188,7 +187,7 @@ class DecodeGraph(StepGraph):
             window = window if 0 <= window < cache.max_seq_len else -1
             C_.decode_qkv_attn(self.qkv, H, Hkv, self.cos, self.sin, cache.cache_seqlens,
                                self.xn if ve is not None else None, w["wg"] if ve is not None else None, ve,
-                               idx if ve is not None else None, kc, vc, window, scale, self.scratch, self.y, table, t_max)
+                               idx if ve is not None else None, kc, vc, window, scale, self.y, table, t_max)
             out = self.x_backout if i == backout_layer else self.xs[i & 1]
             if self.vector:
                 # what the kernel after this layer's last GEMV streams: the next layer's QKV weights, or the head of lm_head

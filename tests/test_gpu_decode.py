@@ -370,22 +370,26 @@ def test_paged_engine_cache_holds_the_prompt_once():
     ops.native_module().check_status()
 
 
-@pytest.mark.parametrize("B,H,Hkv,T,window", [(1, 13, 13, 700, -1), (3, 4, 2, 320, 64), (64, 4, 4, 130, -1), (2, 2, 1, 9000, 4000)])
-def test_fused_append_and_attention_matches_the_two_kernels(B, H, Hkv, T, window):
+@pytest.mark.parametrize("B,H,Hkv,T,window,common", [(1, 13, 13, 700, -1, 0), (3, 4, 2, 320, 64, 0), (64, 4, 4, 130, -1, 0),
+                                                     (2, 2, 1, 9000, 4000, 0), (2, 13, 13, 700, 130, 9), (5, 4, 2, 320, -1, 1), (8, 13, 13, 700, 300, 10),
+                                                     (17, 4, 4, 200, -1, 2), (64, 13, 13, 400, 100, 5), (3, 2, 1, 9000, 4000, 130)])
+def test_fused_append_and_attention_matches_the_two_kernels(B, H, Hkv, T, window, common):
     """Same roundings, other summation order: y is bf16 of float sums over up to 9000 keys, so 2^-8 of a value and what the order of
-    the sums moves (1e-3); the appended token is bitwise the same. Positions at the ends of splits, batches, pages and the window;
+    the sums moves (1e-3). Positions at the ends of splits, batches, pages and the window;
     more pages than the shared-memory table takes (T = 9000)."""
     from nanochat_b200.ops import native as nat
     P, g = 64, torch.Generator(device="cuda").manual_seed(5)
     pages = -(-T // P)
     rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).to(BF16)
     table = torch.randperm(B * pages, device="cuda", generator=g).view(B, pages).to(torch.int32).contiguous()
+    table[:, :common] = table[:1, :common].clone()                       # the first pages are the same for all rows
     k_pool, v_pool = rnd(B * pages + 1, P, Hkv, 128), rnd(B * pages + 1, P, Hkv, 128)
     cos, sin, qkv, xn = rnd(T, 64), rnd(T, 64), rnd(B, (H + 2 * Hkv) * 128), rnd(B, 256)
     wg, ve = torch.randn(Hkv, 12, device="cuda", generator=g), rnd(50, Hkv * 128)
     idx = torch.randint(0, 50, (B,), device="cuda", generator=g)
     scratch = torch.zeros(nat._C.decode_attn_scratch(B, H), dtype=torch.float32, device="cuda")
     for base in (0, 1, 15, 16, 63, 64, 127, T - 1):
+        base = max(base, common * P + B) if common else base             # a row appends to pages of its own
         seqlens = torch.tensor([max(0, min(T - 1, base - b)) for b in range(B)], dtype=torch.int32, device="cuda")
         for gated in (False, True):
             extra = (xn, wg, ve, idx) if gated else (None,) * 4
@@ -394,14 +398,16 @@ def test_fused_append_and_attention_matches_the_two_kernels(B, H, Hkv, T, window
             nat._C.decode_qkv_post(q1, H, Hkv, cos, sin, seqlens, *extra, k1, v1, table, T)
             nat._C.decode_attn(q1[:, :H * 128], k1, v1, seqlens, H, Hkv, window, 0.088, scratch, want, table)
             torch.cuda.synchronize()
-            nat._C.decode_qkv_attn(qkv, H, Hkv, cos, sin, seqlens, *extra, k2, v2, window, 0.088, scratch, got, table, T)
+            nat._C.decode_qkv_attn(qkv, H, Hkv, cos, sin, seqlens, *extra, k2, v2, window, 0.088, got, table, T)
             for a, b in ((k1, k2), (v1, v2)):
-                assert ((a.float() - b.float()).abs() <= 2.0 ** -8 * a.float().abs() + 1e-6).all()
+                # the norm's sum has another order: a value may round to the neighbouring bf16, 2^-7 of it at most, seldom
+                off = (a.float() - b.float()).abs()
+                assert (off <= 2.0 ** -7 * a.float().abs() + 1e-6).all() and (off > 0).sum().item() <= 1e-3 * B * Hkv * 256 + 1
             assert ((got.float() - want.float()).norm() / want.float().norm()).item() < 4e-3, (base, gated)
     full = torch.full((B,), T, dtype=torch.int32, device="cuda")        # a full row: recorded, nothing appended
     k2 = k_pool.clone()
     torch.cuda.synchronize()
-    nat._C.decode_qkv_attn(qkv, H, Hkv, cos, sin, full, None, None, None, None, k2, v_pool, window, 0.088, scratch, got, table, T)
+    nat._C.decode_qkv_attn(qkv, H, Hkv, cos, sin, full, None, None, None, None, k2, v_pool, window, 0.088, got, table, T)
     assert torch.equal(k2, k_pool)
     with pytest.raises(RuntimeError):
         nat.check_status()
