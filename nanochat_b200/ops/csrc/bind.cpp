@@ -370,7 +370,7 @@ void rows_gemm(const Tensor& x, const Tensor& W, const optional<Tensor>& out, co
   };
   nc::RowsGemm g{};
   g.x = x.data_ptr(); g.ldx = x.stride(0); g.W = W.data_ptr(); g.ldw = W.stride(0);
-  g.B = (int)B; g.N = (int)N; g.K = (int)K; g.norm_input = norm_input; g.relu2 = relu2;
+  g.B = (int)B; g.N = (int)N; g.K = (int)K; g.norm_input = norm_input; g.act = relu2 ? nc::ROWS_RELU2 : nc::ROWS_LINEAR; g.overlap = 1;
   if (has(out)) { rows(*out, "out"); g.out = out->data_ptr(); g.ldo = out->stride(0); }
   if (has(aux)) { rows(*aux, "aux"); g.aux = aux->data_ptr(); g.ldaux = aux->stride(0); }
   if (has(xm)) {

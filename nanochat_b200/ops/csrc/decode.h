@@ -35,12 +35,14 @@ cudaError_t gemv_rows_mix(const void* x, long long ldx, const void* x0, long lon
                           void* xm, long long ldxm, void* xn_head, long long ldxn, int head_cols, int B, int N, int K,
                           const void* next_w, long long next_bytes, cudaStream_t s);
 
-// The step's linear layers for up to kRowsGemmMax rows on tensor cores: y = epi(x' W^T) + aux, x' = x or rmsnorm(x)
-// (norm_input), epi = relu^2 where relu2. Any of three results, null for none: out (B x N) bf16; mix.xm = the next layer's
-// stream bf16(lam_r[layer] * bf16(y) + lam_0[layer] * x0); logits (B x N) fp32 = softcap * tanh(y / softcap).
+// Linear layers for up to kRowsGemmMax rows on tensor cores: y = act(x' W^T) + aux (times aux with mul_aux), x' = x or
+// rmsnorm(x) (norm_input). Any of three results, null for none: out (B x N) bf16; mix.xm = the next layer's stream
+// bf16(lam_r[layer] * bf16(y) + lam_0[layer] * x0); logits (B x N) fp32 = softcap * tanh(y / softcap), y itself with softcap 0.
 // xn_head: with norm_input, the first head_cols (<= 128) channels of rmsnorm(x). K, ldx, ldw multiples of 8, x and W
-// 16-byte aligned. W is read before the wait on the kernel in front, which must not be the one that wrote it.
+// 16-byte aligned. overlap: the kernel may start while the one in front ends; it then reads W before the wait on that kernel,
+// which must not be the one that wrote it.
 constexpr int kRowsGemmMax = 64;
+enum RowsAct : int { ROWS_LINEAR = 0, ROWS_RELU2 = 1, ROWS_RELU = 2 };
 struct RowsMix {
   const float* lam_r = nullptr; const float* lam_0 = nullptr; int layer = 0;
   const __nv_bfloat16* x0 = nullptr; long long ldx0 = 0;
@@ -48,12 +50,12 @@ struct RowsMix {
 };
 struct RowsGemm {
   const void* x; long long ldx; const void* W; long long ldw; int B, N, K;
-  int norm_input = 0, relu2 = 0;
+  int norm_input = 0, act = ROWS_LINEAR, mul_aux = 0, overlap = 0;
   const void* aux = nullptr; long long ldaux = 0;
   void* out = nullptr; long long ldo = 0;
   RowsMix mix;
   void* xn_head = nullptr; long long ldxn = 0; int head_cols = 0;
-  float* logits = nullptr; long long ldl = 0; float softcap = 1.f;
+  float* logits = nullptr; long long ldl = 0; float softcap = 0.f;
   int* status = nullptr;
 };
 cudaError_t rows_gemm(const RowsGemm& g, cudaStream_t s);

@@ -18,6 +18,7 @@
 // (one elected lane), warps 2..9 = epilogue (a warp may read the TMEM lane quadrant
 // warp_id % 4; the two warps of a quadrant take one half of the tile's columns each). All waits are bounded (ptx.cuh); a failed wait raises the CTA abort
 // flag, records a status word and the kernel drains and exits normally.
+#include "decode.h"
 #include "gemm.h"
 #include "host_utils.cuh"
 #include "ptx.cuh"
@@ -1286,11 +1287,33 @@ cudaError_t symmetrize_bf16(void* C, int n, long long ld, long long bs, int batc
   return cudaGetLastError();
 }
 
+// Up to 64 rows against K-major weights: the kernel that makes the weights the 128-row operand and splits K (rows_gemm.cu); here
+// they would fill a fraction of a 128-row tile and one SM per tile of columns would read all of its weights. 16 rows, B200:
+// 1664 x 6656 24 us here and 6 there, 32768 x 1664 30 / 20.
+static bool rows_form(const GemmDesc& d) {
+  return d.M <= kRowsGemmMax && !d.a_mn && !d.b_mn && d.batch == 1 && d.bn == 0 && d.pair < 0 && !d.symmetric && d.m_group == nullptr &&
+         d.alpha == 1.f && d.scale_a == nullptr && d.scale_b == nullptr && d.amax_out == nullptr && (d.K & 7) == 0 &&
+         ((reinterpret_cast<uintptr_t>(d.A) | reinterpret_cast<uintptr_t>(d.B)) & 15) == 0 &&
+         (d.epi == EPI_LINEAR ? d.aux == nullptr || d.beta == 0.f || (!d.c_f32 && d.beta == 1.f)
+                              : !d.c_f32 && (d.epi == EPI_RELU2 || d.epi == EPI_RELU || (d.epi == EPI_MULAUX && d.aux != nullptr)));
+}
+static cudaError_t gemm_rows(const GemmDesc& d, int* status, cudaStream_t stream) {
+  RowsGemm g{};
+  g.x = d.A; g.ldx = d.lda; g.W = d.B; g.ldw = d.ldb; g.B = d.M; g.N = d.N; g.K = d.K;
+  g.act = d.epi == EPI_RELU2 ? ROWS_RELU2 : d.epi == EPI_RELU ? ROWS_RELU : ROWS_LINEAR;
+  if (d.epi == EPI_MULAUX || (d.epi == EPI_LINEAR && d.aux != nullptr && d.beta != 0.f)) { g.aux = d.aux; g.ldaux = d.ldaux; }
+  g.mul_aux = d.epi == EPI_MULAUX;
+  if (d.c_f32) { g.logits = reinterpret_cast<float*>(d.C); g.ldl = d.ldc; } else { g.out = d.C; g.ldo = d.ldc; }
+  g.status = status;
+  return rows_gemm(g, stream);
+}
+
 cudaError_t gemm_bf16(const GemmDesc& d, int* status, cudaStream_t stream) {
   if (d.M <= 0 || d.N <= 0 || d.K <= 0 || d.batch <= 0) return cudaErrorInvalidValue;
   if ((d.N & 7) || (d.lda & 7) || (d.ldb & 7) || (d.ldc & 3)) return cudaErrorInvalidValue;
   if (d.m_group && (d.groups <= 0 || d.batch != 1 || d.a_mn || d.b_mn || d.symmetric || (d.bsb & 7) || d.pair > 0 || d.aux))
     return cudaErrorInvalidValue;
+  if (rows_form(d)) return gemm_rows(d, status, stream);
   const GemmPlan p = gemm_plan(d, false);
   if (best_is_invalid(p, d)) return cudaErrorInvalidValue;
   return launch_major<false>(p.bn, p.pair, d, status, stream);

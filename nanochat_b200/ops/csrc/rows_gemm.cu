@@ -1,4 +1,4 @@
-// Linear layers of a decode step of up to 64 rows on the 5th-generation tensor cores:
+// Linear layers of up to 64 rows (decode steps, short prompts) on the 5th-generation tensor cores:
 //
 //   y[b, n] = epi( sum_k x'[b, k] W[n, k] ) + aux[b, n],   x' = x or rmsnorm(x)
 //
@@ -43,7 +43,7 @@ struct Cfg {
 };
 
 struct Args {
-  int B, N, K, splits, norm_input, relu2, head_cols;
+  int B, N, K, splits, norm_input, act, mul_aux, head_cols;
   const __nv_bfloat16* aux; long long ldaux;
   __nv_bfloat16* out; long long ldo;
   RowsMix mix;
@@ -220,14 +220,18 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             v *= rstd;
             if (head) a.xn_head[b * a.ldxn + n] = __float2bfloat16(__bfloat162float(a.x[b * a.ldx + n]) * rstd);
           }
-          if (a.relu2) { v = fmaxf(v, 0.f); v *= v; }
-          if (a.aux != nullptr) v += __bfloat162float(a.aux[b * a.ldaux + n]);
+          if (a.act != ROWS_LINEAR) v = fmaxf(v, 0.f);
+          if (a.act == ROWS_RELU2) v *= v;
+          if (a.aux != nullptr) {
+            const float x = __bfloat162float(a.aux[b * a.ldaux + n]);
+            v = a.mul_aux ? v * x : v + x;
+          }
           if (a.out != nullptr) a.out[b * a.ldo + n] = __float2bfloat16(v);
           if (mix) {
             const float x0 = __bfloat162float(a.mix.x0[b * a.mix.ldx0 + n]);
             a.mix.xm[b * a.mix.ldxm + n] = __float2bfloat16(lam_r * round_bf16(v) + lam_0 * x0);
           }
-          if (a.logits != nullptr) a.logits[b * a.ldl + n] = a.softcap * tanhf(v / a.softcap);
+          if (a.logits != nullptr) a.logits[b * a.ldl + n] = a.softcap > 0.f ? a.softcap * tanhf(v / a.softcap) : v;
         }
       }
     }
@@ -247,7 +251,7 @@ rows_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 }
 
 template <int R>
-cudaError_t launch(const CUtensorMap& tmW, const CUtensorMap& tmX, const Args& a, cudaStream_t s) {
+cudaError_t launch(const CUtensorMap& tmW, const CUtensorMap& tmX, const Args& a, bool overlap, cudaStream_t s) {
   static PerDeviceOnce configured;
   cudaError_t e = configured.once([] {
     return cudaFuncSetAttribute(rows_gemm_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<R>::SMEM);
@@ -256,11 +260,11 @@ cudaError_t launch(const CUtensorMap& tmW, const CUtensorMap& tmX, const Args& a
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((a.N + BM - 1) / BM * a.splits); cfg.blockDim = dim3(THREADS); cfg.dynamicSmemBytes = Cfg<R>::SMEM; cfg.stream = s;
   cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = a.splits; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
-  cfg.attrs = at; cfg.numAttrs = 2;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = a.splits; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at; cfg.numAttrs = overlap ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, rows_gemm_kernel<R>, tmW, tmX, a);
 }
 
@@ -277,7 +281,7 @@ cudaError_t rows_gemm(const RowsGemm& g, cudaStream_t s) {
   int splits = 1;
   while (splits < MAX_SPLIT && tiles * splits < sm_count() && 2 * splits <= blocks) splits *= 2;
   Args a = {};
-  a.B = g.B; a.N = g.N; a.K = g.K; a.splits = splits; a.norm_input = g.norm_input; a.relu2 = g.relu2;
+  a.B = g.B; a.N = g.N; a.K = g.K; a.splits = splits; a.norm_input = g.norm_input; a.act = g.act; a.mul_aux = g.mul_aux;
   a.aux = reinterpret_cast<const __nv_bfloat16*>(g.aux); a.ldaux = g.ldaux;
   a.out = reinterpret_cast<__nv_bfloat16*>(g.out); a.ldo = g.ldo;
   a.mix = g.mix;
@@ -292,7 +296,8 @@ cudaError_t rows_gemm(const RowsGemm& g, cudaStream_t s) {
   if (!make_tmap(&tmW, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, g.W, wd, ws, wb) ||
       !make_tmap(&tmX, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, g.x, xd, xs, xb))
     return cudaErrorInvalidValue;
-  return R == 16 ? launch<16>(tmW, tmX, a, s) : R == 32 ? launch<32>(tmW, tmX, a, s) : launch<64>(tmW, tmX, a, s);
+  const bool o = g.overlap != 0;
+  return R == 16 ? launch<16>(tmW, tmX, a, o, s) : R == 32 ? launch<32>(tmW, tmX, a, o, s) : launch<64>(tmW, tmX, a, o, s);
 }
 
 }  // namespace nc

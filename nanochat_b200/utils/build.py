@@ -107,7 +107,7 @@ def cuda_sources():
 
 
 def serving_sources():
-    shared = [os.path.join(CSRC, f) for f in ("attention.cu", "gemm.cu")]
+    shared = [os.path.join(CSRC, f) for f in ("attention.cu", "gemm.cu", "rows_gemm.cu")]
     return (sorted(glob.glob(os.path.join(SERVE_CSRC, "*.cu"))) + shared, sorted(glob.glob(os.path.join(SERVE_CSRC, "*.cpp"))))
 
 

@@ -166,3 +166,22 @@ def test_fused_epilogues_with_an_auxiliary_operand(nat, M, N, K, bn, b_mn, pair)
     nat.gemm(A, B, inplace, aux=inplace, beta=1.0, **kw)
     nat.check_status(inplace)
     assert _rel_err(inplace, prod + aux.float()) < 1e-2
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (5, 136, 200), (45, 2304, 768), (64, 1664, 6656), (65, 520, 136)])
+def test_few_rows_against_k_major_weights(nat, M, N, K):
+    """Up to 64 rows another kernel takes the product; bf16 results are off by at most 2^-9 of a value, fp32 ones by the order of the
+    sum (K * 2^-24 at worst, far less in the norm)."""
+    A, B, aux = _mk((M, K), seed=1).to(BF16), _mk((N, K), K ** -0.5, seed=2).to(BF16), _mk((M, N), seed=3).to(BF16)
+    ref = A.float() @ B.float().t()
+    wide = torch.zeros(M, N + 8, dtype=BF16, device="cuda")
+    out = wide[:, :N]                                        # a row pitch of its own
+    for kw, want in ((dict(), ref), (dict(epi=nat.EPI_RELU2), torch.relu(ref) ** 2), (dict(epi=nat.EPI_RELU), torch.relu(ref)),
+                     (dict(aux=aux, beta=1.0), ref + aux.float()), (dict(aux=aux, epi=nat.EPI_MULAUX), ref * aux.float())):
+        nat.gemm(A, B, out, **kw)
+        assert _rel_err(out, want) < 4e-3, kw
+        assert wide[:, N:].abs().sum().item() == 0
+    whole = torch.empty(M, N, device="cuda")
+    nat.gemm(A, B, whole)
+    assert _rel_err(whole, ref) < 1e-5
+    nat.check_status()
