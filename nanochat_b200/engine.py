@@ -474,8 +474,12 @@ class Engine:
         """Run a portion of tokens; (len(want), V) logits at the places `want`, None when there are none."""
         if self.own_cache:
             return self.model.forward(ids, kv_cache=cache, want=list(want))
-        logits = self.model.forward(ids, kv_cache=cache)[0]
-        return logits[list(want)].float() if len(want) else None
+        from nanochat_b200.models.gpt import GPT
+        if not isinstance(self.model, GPT):
+            logits = self.model.forward(ids, kv_cache=cache)[0]
+            return logits[list(want)].float() if len(want) else None
+        logits = self.model.forward(ids, kv_cache=cache, want=list(want))
+        return None if logits is None else logits[0].float()
 
     def _begin_decode(self, cache):
         """The cache has been filled by a prompt: let its captured decode step take over what the prompt left."""

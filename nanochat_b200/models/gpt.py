@@ -333,7 +333,10 @@ class GPT(nn.Module, NaiveSampler):
             x = x + gate * prev
         return x
 
-    def forward(self, idx, targets=None, kv_cache=None, loss_reduction="mean"):
+    def forward(self, idx, targets=None, kv_cache=None, loss_reduction="mean", want=None):
+        """`want`: positions whose logits a prompt into a cache returns, (B, len(want), V), None when there are none."""
+        if want is not None and (targets is not None or kv_cache is None):
+            raise ValueError("want picks logits of a prompt")
         B, T = idx.size()
         assert T <= self.cos.size(1), f"Sequence length grew beyond the rotary embeddings cache: {T} > {self.cos.size(1)}"
         assert idx.device == self.cos.device, f"Rotary embeddings and idx are on different devices: {idx.device} != {self.cos.device}"
@@ -348,8 +351,9 @@ class GPT(nn.Module, NaiveSampler):
         if (kv_cache is not None and T > 1 and T0 == 0 and kv_cache.prev_embedding is None
                 and not torch.is_grad_enabled() and common.COMPUTE_DTYPE == torch.bfloat16
                 and self.config.n_embd // self.config.n_head == 128 and T <= kv_cache.max_seq_len
-                and ops.use_native(self.transformer.wte.weight)):
-            return self._prefill_native(idx, cos_sin, kv_cache)
+                and ops.use_native(self.transformer.wte.weight) and ops.native_module().ATTENTION_IMPL == "native"
+                and all(c.dtype == torch.bfloat16 for c in kv_cache.get_layer_cache(0))):
+            return self._prefill_native(idx, cos_sin, kv_cache, want)
 
         x = self._embed(idx, kv_cache)
         x0 = x
@@ -369,6 +373,10 @@ class GPT(nn.Module, NaiveSampler):
             if loss_reduction == "none":
                 loss = loss.view(-1)
             return loss
+        if want is not None:
+            if not want:
+                return None
+            x = x[:, want]
         return ops.softcap_logits(x, self.lm_head.weight, self.config.vocab_size)
 
     def _forward_native(self, idx, targets, cos_sin, loss_reduction):
@@ -398,23 +406,36 @@ class GPT(nn.Module, NaiveSampler):
         x = ops.backout_norm(x, x_backout, self.backout_lambda)
         return nat.softcap_logits(x, self.lm_head.weight, self.config.vocab_size)
 
-    def _prefill_native(self, idx, cos_sin, kv_cache):
-        """Prompt into an empty cache on the fused per-layer path of training (one QKV GEMM, rotary / QK-norm / VE
-        gate in place, the whole-sequence attention kernel), each layer's keys and values copied into its cache.
-        The op-by-op cached forward launches about twice as many kernels and is bound by their launch cost."""
+    def _prefill_native(self, idx, cos_sin, kv_cache, want=None):
+        """Prompt into an empty cache: the kernels of the training forward, launched for all layers from one native call that
+        leaves each layer's keys and values in its cache. Logits of every position, or (B, len(want), V) of those in `want`."""
         nat = ops.native_module()
-        T = idx.size(1)
-        x, last = nat.embed_norm_smear(idx, self.transformer.wte.weight, self.smear_gate.weight, self.smear_lambda)
+        cfg, (B, T) = self.config, idx.shape
+        idx = idx.long().contiguous()
+        x0, last = nat.embed_norm_smear(idx, self.transformer.wte.weight, self.smear_gate.weight, self.smear_lambda)
         kv_cache.prev_embedding = last
-        x0 = x
-        backout_layer = self.config.n_layer // 2
-        x_backout = None
+        weights, gates, tables, sinks = [], [], [], []
         for i, block in enumerate(self.transformer.h):
-            ve_w = self.value_embeds[str(i)].weight if str(i) in self.value_embeds else None
-            x = nat.layer_forward(block, x, x0, idx, ve_w, cos_sin, self.window_sizes[i],
-                                  self.resid_lambdas, self.x0_lambdas, i, kv_sink=kv_cache.get_layer_cache(i))
-            if i == backout_layer:
-                x_backout = x
+            a, mlp = block.attn, block.mlp
+            weights.append([nat.shadow_of(w).contiguous() for w in (a.c_q.weight, a.c_k.weight, a.c_v.weight, a.c_proj.weight,
+                                                                    mlp.c_fc.weight, mlp.c_proj.weight)])
+            gates.append(None if a.ve_gate is None else a.ve_gate.weight.detach().float().contiguous())
+            tables.append(self.value_embeds[str(i)].weight if str(i) in self.value_embeds else None)
+            sinks.append(kv_cache.get_layer_cache(i))
+        x, x_backout = nat._C.gpt_prefill(x0.contiguous(), idx, cos_sin[0].reshape(-1, 64), cos_sin[1].reshape(-1, 64), self.resid_lambdas,
+                                          self.x0_lambdas, weights, gates, tables, [k for k, _ in sinks], [v for _, v in sinks],
+                                          [w[0] for w in self.window_sizes], cfg.n_head, cfg.n_kv_head, cfg.n_layer // 2)
         kv_cache.advance(T)
-        x = ops.backout_norm(x, x_backout, self.backout_lambda)
-        return nat.softcap_logits(x, self.lm_head.weight, self.config.vocab_size)
+        x, x_backout = x.view(B, T, -1), x_backout.view(B, T, -1)
+        if want is not None and not want:
+            return None
+        lm_head = nat.shadow_of(self.lm_head.weight)[:cfg.vocab_size]     # cast, if at all, well ahead of its product
+        if want is not None:
+            x, x_backout = x[:, want].contiguous(), x_backout[:, want].contiguous()
+        xn = torch.empty_like(x)
+        nat._C.backout_norm_fwd(x, x_backout, self.backout_lambda.detach().float(), xn)
+        if xn.shape[0] * xn.shape[1] <= 64:
+            logits = torch.empty(xn.shape[0] * xn.shape[1], cfg.vocab_size, dtype=torch.float32, device=xn.device)
+            nat._C.rows_gemm(xn.view(-1, xn.shape[2]), lm_head, logits=logits, softcap=ref_ops.SOFTCAP)
+            return logits.view(xn.shape[0], xn.shape[1], cfg.vocab_size)
+        return nat.softcap_logits(xn, self.lm_head.weight, cfg.vocab_size)

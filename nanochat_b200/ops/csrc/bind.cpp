@@ -11,6 +11,7 @@
 #include "decode.h"
 #include "gemm.h"
 #include "optim.h"
+#include "prefill.h"
 
 namespace {
 
@@ -354,6 +355,71 @@ void gemv_rows_mix(const Tensor& x, const Tensor& x0, const Tensor& lam_r, const
                              (int)x.size(1), next_weights(next_w).first, next_weights(next_w).second, cur_stream()));
 }
 
+// GPT's layers over a prompt. x0: (B, T, C) bf16, idx: (B, T) int64, cos / sin: (T, 64). Per layer: weights = [q, k, v, o, fc, pr]
+// (bf16, dense), gates fp32 (Hkv, 12) and ve bf16 (V, Hkv * 128) or None, sinks k and v (B, >= T, Hkv, 128), windows.
+// Returns (last layer's output, backout layer's output), (B * T, C).
+std::pair<Tensor, Tensor> gpt_prefill(const Tensor& x0, const Tensor& idx, const Tensor& cos_t, const Tensor& sin_t, const Tensor& lam_r,
+                                      const Tensor& lam_0, const std::vector<std::vector<Tensor>>& weights,
+                                      const std::vector<optional<Tensor>>& gates, const std::vector<optional<Tensor>>& ves,
+                                      const std::vector<Tensor>& k_sinks, const std::vector<Tensor>& v_sinks,
+                                      const std::vector<int64_t>& windows, int64_t H, int64_t Hkv, int64_t backout_layer) {
+  check_bf16(x0, "x0"); check_bf16(cos_t, "cos"); check_bf16(sin_t, "sin");
+  const size_t n = weights.size();
+  TORCH_CHECK(x0.dim() == 3 && x0.is_contiguous() && idx.is_cuda() && idx.scalar_type() == at::kLong && idx.is_contiguous() &&
+              idx.numel() == x0.size(0) * x0.size(1), "gpt_prefill: x0 (B, T, C), idx int64 (B, T)");
+  const int64_t B = x0.size(0), T = x0.size(1), C = x0.size(2), nq = H * 128, nkv = Hkv * 128;
+  TORCH_CHECK(cos_t.is_contiguous() && sin_t.is_contiguous() && cos_t.numel() >= T * 64 && sin_t.numel() >= T * 64 && cos_t.size(-1) == 64, "rotary tables");
+  TORCH_CHECK(n > 0 && gates.size() == n && ves.size() == n && k_sinks.size() == n && v_sinks.size() == n && windows.size() == n &&
+              backout_layer >= 0 && backout_layer < (int64_t)n && C % 8 == 0 && C >= 16, "gpt_prefill: one entry per layer");
+  for (const Tensor* t : {&lam_r, &lam_0})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() >= (int64_t)n, "lambdas: fp32 (layers)");
+  const int64_t ff = weights[0][4].size(0);
+  const Tensor& s0 = k_sinks[0];
+  std::vector<nc::PrefillLayer> layers(n);
+  for (size_t i = 0; i < n; ++i) {
+    TORCH_CHECK(weights[i].size() == 6, "gpt_prefill: six matrices per layer");
+    const int64_t rows[6] = {nq, nkv, nkv, C, ff, C}, cols[6] = {C, C, C, nq, C, ff};
+    for (int k = 0; k < 6; ++k) {
+      const Tensor& w = weights[i][k];
+      check_bf16(w, "weight");
+      TORCH_CHECK(w.dim() == 2 && w.is_contiguous() && w.size(0) == rows[k] && w.size(1) == cols[k], "gpt_prefill: weight shape");
+    }
+    for (const Tensor* t : {&k_sinks[i], &v_sinks[i]}) {
+      check_bf16(*t, "sink");
+      TORCH_CHECK(t->dim() == 4 && t->size(0) == B && t->size(1) >= T && t->size(2) == Hkv && t->size(3) == 128 && t->strides() == s0.strides() &&
+                  t->stride(3) == 1 && t->stride(2) == 128 && t->stride(1) % 8 == 0 && t->stride(0) % 8 == 0 &&
+                  reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "gpt_prefill: cache layout");
+    }
+    nc::PrefillLayer& l = layers[i];
+    l = {weights[i][0].data_ptr(), weights[i][1].data_ptr(), weights[i][2].data_ptr(), weights[i][3].data_ptr(), weights[i][4].data_ptr(),
+         weights[i][5].data_ptr(), nullptr, nullptr, k_sinks[i].data_ptr(), v_sinks[i].data_ptr(), (int)windows[i]};
+    if (ves[i].has_value() && ves[i]->defined()) {
+      const Tensor &ve = *ves[i], &wg = *gates[i];
+      check_bf16(ve, "ve");
+      TORCH_CHECK(ve.dim() == 2 && ve.is_contiguous() && ve.size(1) == nkv && wg.scalar_type() == at::kFloat && wg.is_contiguous() &&
+                  wg.numel() == Hkv * 12, "gpt_prefill: value embedding");
+      l.ve = ve.data_ptr(); l.wg = wg.data_ptr<float>();
+    }
+  }
+  const c10::cuda::CUDAGuard guard(x0.device());
+  const int64_t M = B * T;
+  auto rows = [&](int64_t width) { return at::empty({M, width}, x0.options()); };
+  const auto f32 = x0.options().dtype(at::kFloat);
+  Tensor xm = rows(C), xn = rows(C), xa = rows(C), xs0 = rows(C), xs1 = rows(C), back = rows(C), y = rows(nq), qkv = rows(nq + 2 * nkv), h = rows(ff);
+  Tensor rstd = at::empty({M, H + Hkv}, f32), lse = at::empty({B, H, T}, f32);
+  nc::Prefill p{};
+  p.B = (int)B; p.T = (int)T; p.C = (int)C; p.H = (int)H; p.Hkv = (int)Hkv; p.ff = (int)ff; p.layers = (int)n; p.backout_layer = (int)backout_layer;
+  p.x0 = x0.data_ptr(); p.idx = reinterpret_cast<const long long*>(idx.data_ptr<int64_t>());
+  p.cos_t = cos_t.data_ptr(); p.sin_t = sin_t.data_ptr(); p.lam_r = lam_r.data_ptr<float>(); p.lam_0 = lam_0.data_ptr<float>();
+  p.scale = (float)(1.0 / std::sqrt(128.0)); p.sink_bat = s0.stride(0); p.sink_tok = s0.stride(1);
+  p.xm = xm.data_ptr(); p.xn = xn.data_ptr(); p.xa = xa.data_ptr(); p.x[0] = xs0.data_ptr(); p.x[1] = xs1.data_ptr(); p.x_backout = back.data_ptr();
+  p.y = y.data_ptr(); p.qkv = qkv.data_ptr(); p.h = h.data_ptr(); p.rstd = rstd.data_ptr<float>(); p.lse = lse.data_ptr<float>();
+  p.status = status_ptr(x0);
+  NC_CHECK(nc::gpt_prefill(p, layers.data(), cur_stream()));
+  const int64_t last = (int64_t)n - 1;
+  return {last == backout_layer ? back : (last & 1 ? xs1 : xs0), back};
+}
+
 // x: (B, K), W: (N, K), out / aux: (B, N) bf16; x0, xm: (B, N) bf16 with lam_r, lam_0 fp32 (layers); xn: (B, K) bf16, its first
 // 16 channels are written; logits: fp32 (B, N).
 void rows_gemm(const Tensor& x, const Tensor& W, const optional<Tensor>& out, const optional<Tensor>& aux, bool relu2,
@@ -694,6 +760,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("relu2") = false, py::arg("norm_input") = false, py::arg("x0") = py::none(), py::arg("lam_r") = py::none(),
         py::arg("lam_0") = py::none(), py::arg("layer") = 0, py::arg("xm") = py::none(), py::arg("xn") = py::none(),
         py::arg("logits") = py::none(), py::arg("softcap") = 1.0);
+  m.def("gpt_prefill", &gpt_prefill);
   m.def("decode_embed", &decode_embed);
   m.def("decode_qkv_post", &decode_qkv_post, py::arg("qkv"), py::arg("H"), py::arg("Hkv"), py::arg("cos"), py::arg("sin"),
         py::arg("seqlens"), py::arg("xn"), py::arg("wg"), py::arg("ve"), py::arg("idx"), py::arg("k_cache"),

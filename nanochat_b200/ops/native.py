@@ -607,7 +607,7 @@ class _LayerFn(Function):
 
     @staticmethod
     def forward(ctx, x, x0, idx, cos, sin, resid_lambdas, x0_lambdas, layer, wq, wk, wv, wo, wfc, wpr,
-                wgate, ve_w, window, n_head, n_kv_head, kv_sink=None, x0_pass=(0, True)):
+                wgate, ve_w, window, n_head, n_kv_head, x0_pass=(0, True)):
         B, T, C = x.shape
         M = B * T
         D = C // n_head
@@ -618,8 +618,7 @@ class _LayerFn(Function):
         nq, nkv = n_head * D, n_kv_head * D
         sq, sk, sv = shadow_of(wq), shadow_of(wk), shadow_of(wv)
         fused_w = _contiguous_rows([sq, sk, sv])
-        # kv_sink: (k_cache, v_cache) of this layer, (B, Tmax, Hkv, D): prefill of an empty cache (inference, bf16)
-        fp8 = kv_sink is None and fused_w is not None and _fp8_ok(C, nq, nkv, wfc.shape[0])
+        fp8 = fused_w is not None and _fp8_ok(C, nq, nkv, wfc.shape[0])
         # producers that hold whole rows report max|output| themselves: no separate pass for the fp8 scale
         amax_xn = _zeroed_scalar(dev) if fp8 else None
         _C.mixnorm_fwd(x2, x02, resid_lambdas, x0_lambdas, layer, xm, xn, amax_xn)
@@ -648,9 +647,6 @@ class _LayerFn(Function):
         q = qkv[:, :nq].view(B, T, n_head, D)
         k = qkv[:, nq:nq + nkv].view(B, T, n_kv_head, D)
         v = qkv[:, nq + nkv:].view(B, T, n_kv_head, D)
-        if kv_sink is not None:
-            kv_sink[0][:, :T].copy_(k)
-            kv_sink[1][:, :T].copy_(v)
         amax_y = _zeroed_scalar(dev) if fp8 else None
         y, lse = attention_forward(q, k, v, window, amax_y)
         if lse is None:
@@ -835,12 +831,12 @@ class _LayerFn(Function):
             _amax_hints[dx.data_ptr()] = amax_dx
         if not owns_pass:
             _dx0_running[pass_id] = dx0
-            return (dx.view(B, T, C), None) + (None,) * 19
+            return (dx.view(B, T, C), None) + (None,) * 18
         _x0_open.discard(pass_id)
-        return (dx.view(B, T, C), dx0.view(B, T, C)) + (None,) * 19
+        return (dx.view(B, T, C), dx0.view(B, T, C)) + (None,) * 18
 
 
-def layer_forward(block, x, x0, idx, ve_weight, cos_sin, window_size, resid_lambdas, x0_lambdas, layer, kv_sink=None):
+def layer_forward(block, x, x0, idx, ve_weight, cos_sin, window_size, resid_lambdas, x0_lambdas, layer):
     attn, mlp = block.attn, block.mlp
     pass_id, owns_pass = 0, True
     if torch.is_grad_enabled() and x0.requires_grad:
@@ -858,7 +854,7 @@ def layer_forward(block, x, x0, idx, ve_weight, cos_sin, window_size, resid_lamb
         attn.c_q.weight, attn.c_k.weight, attn.c_v.weight, attn.c_proj.weight,
         mlp.c_fc.weight, mlp.c_proj.weight,
         attn.ve_gate.weight if ve_weight is not None else None, ve_weight,
-        window_size[0], attn.n_head, attn.n_kv_head, kv_sink, (pass_id, owns_pass))
+        window_size[0], attn.n_head, attn.n_kv_head, (pass_id, owns_pass))
 
 
 # ------------------------------------------------------------------------ head function

@@ -411,3 +411,24 @@ def test_fused_append_and_attention_matches_the_two_kernels(B, H, Hkv, T, window
     assert torch.equal(k2, k_pool)
     with pytest.raises(RuntimeError):
         nat.check_status()
+
+
+@pytest.mark.parametrize("tokens", [2, 63, 64, 65, 200])
+def test_prompt_in_one_call_matches_the_op_by_op_forward(tokens):
+    """Logits of wanted and of all positions, keys and values: against the same weights without a cache, where every layer runs as
+    the training forward does. Two bf16 forwards of four layers; the switch to the few-row products lies at 64 tokens."""
+    from nanochat_b200.engine import KVCache
+    model = _model()
+    cfg = model.config
+    ids = torch.randint(0, cfg.vocab_size, (1, tokens), device="cuda", generator=torch.Generator(device="cuda").manual_seed(tokens))
+    mk = lambda: KVCache(batch_size=1, num_heads=cfg.n_kv_head, seq_len=256, head_dim=128, num_layers=cfg.n_layer, device="cuda", dtype=BF16)
+    with torch.inference_mode():
+        want = model.forward(ids)
+        a, b, c = mk(), mk(), mk()
+        every, some = model.forward(ids, kv_cache=a), model.forward(ids, kv_cache=b, want=[tokens - 1, 0])
+        assert model.forward(ids, kv_cache=c, want=[]) is None and c.get_pos() == tokens
+        close = lambda x, y: ((x.float() - y.float()).norm() / y.float().norm()).item() < 2e-2
+        assert close(every, want) and close(some, want[:, [tokens - 1, 0]])
+        for layer in range(cfg.n_layer):
+            for x, y in zip(a.get_layer_cache(layer), b.get_layer_cache(layer)):
+                assert torch.equal(x, y) and x[:, tokens:].abs().sum().item() == 0 and (x[:, :tokens].abs().sum(-1) > 0).all()
